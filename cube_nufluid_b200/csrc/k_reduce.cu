@@ -430,7 +430,10 @@ __global__ void __launch_bounds__(1024) k_vdec_build(const float* __restrict__ t
 const double* cube_vdec_table(cube_ctx* ctx, double coef, int* rc) {
   *rc = CUBE_OK;
   for (int i = 0; i < 2; ++i)
-    if (ctx->vdec[i] && ctx->vdec_coef[i] == coef) return ctx->vdec[i];
+    if (ctx->vdec[i] && ctx->vdec_coef[i] == coef) {
+      ctx->vdec_next = i ^ 1;  // the caller may ask for another beside it (the kick decodes by two)
+      return ctx->vdec[i];
+    }
   const int i = ctx->vdec_next;
   ctx->vdec_next ^= 1;
   if (!ctx->vdec[i] && cudaMalloc((void**)&ctx->vdec[i], sizeof(double) * ctx->nvbin + sizeof(uint32_t) * (ctx->nvbin / 32) + 64) !=
