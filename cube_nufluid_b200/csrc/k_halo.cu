@@ -808,7 +808,9 @@ std::vector<int> halo_waves(const std::vector<HaloCand>& hc, const std::vector<d
   double rmax = 0.0;
   for (double r : rs) rmax = std::max(rmax, r);
   const double reach = 2.0 * rmax + 1e-6;
-  const int G = std::max(1, (int)std::floor(nf / std::max(reach, 1e-9)));  // buckets per dimension
+  // buckets per dimension: at least reach wide, and about one per candidate at most (without
+  // a candidate reach is nothing, and the buckets it asks for would be without number)
+  const int G = std::max(1, (int)std::min(std::floor(nf / reach), std::ceil(std::cbrt((double)n))));
   const double bw = (double)nf / G;
   std::vector<std::vector<int>> bucket((size_t)G * G * G);
   auto bidx = [&](double x) { int b = (int)std::floor(x / bw); return ((b % G) + G) % G; };

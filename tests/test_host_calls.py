@@ -1,0 +1,60 @@
+"""What the library's host code does around its launches, on the CPU: the library runs in a
+child process over a recording CUDA runtime on host memory (fake_cudart.cpp), whose
+kernels do nothing, and the test reads the calls that it made.
+"""
+import json
+import os
+import subprocess
+import sys
+
+import pytest
+
+TESTS = os.path.dirname(os.path.abspath(__file__))
+ROOT = os.path.dirname(TESTS)
+CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
+
+CHILD = """
+import ctypes as C, json, os, sys
+import numpy as np
+sys.path.insert(0, {root!r})
+from cube_nufluid_b200 import Cube, CubeError
+from cube_nufluid_b200.abi import CubeScalars, make_params
+fake = C.CDLL(os.environ["LD_PRELOAD"])
+fake.fake_log.restype = C.c_char_p
+fake.fake_poke.argtypes = [C.c_size_t, C.c_size_t, C.c_ulonglong]
+
+def calls():
+    return [dict(zip(("call", "name", "src", "stream"), l.split())) for l in fake.fake_log().decode().splitlines()]
+
+def empty_box():
+    g = Cube(make_params(16, 2), np_capacity=64)
+    g.load_state(np.zeros((0, 3), np.int16), np.zeros((0, 3), np.int16), np.zeros(0, np.int32),
+                 np.zeros(16 ** 3, np.int32), np.zeros((16 ** 3, 3), np.float32))
+    return g
+"""
+
+
+@pytest.fixture(scope="module")
+def child(tmp_path_factory):
+    """runs code after CHILD and returns the JSON it prints"""
+    so = str(tmp_path_factory.mktemp("fake") / "libfake_cudart.so")
+    subprocess.run(["g++", "-O1", "-shared", "-fPIC", f"-I{CUDA}/include", "-o", so, os.path.join(TESTS, "fake_cudart.cpp")],
+                   check=True)
+
+    def run(code):
+        r = subprocess.run([sys.executable, "-c", CHILD.format(root=ROOT) + code], env=dict(os.environ, LD_PRELOAD=so),
+                           capture_output=True, text=True, timeout=120)
+        assert r.returncode == 0, r.stderr[-2000:]
+        return json.loads(r.stdout)
+
+    return run
+
+
+def test_halofind_of_a_box_without_peaks(child):
+    assert child("""
+g = empty_box()
+s = CubeScalars()
+s.a, s.sigma_vi, s.mass_p_cdm, s.vsim2phys = 0.5, 0.01, 1.0, 1.0
+halos, members, hid, npeak = g.halofind(s, hid_len=10)
+print(json.dumps([len(halos), len(members), hid.tolist(), npeak]))
+""") == [0, 0, [0] * 10, 0]
