@@ -878,7 +878,8 @@ int run_halofind(cube_ctx* ctx, const cube_scalars* io, const cube_halo_args* ha
   if (!ctx->halo_shells) {  // 18 MB, kept by the context
     int4* q = nullptr;
     CUBE_CUDA_TRY(ctx, cudaMalloc((void**)&q, sizeof(int4) * sl.size()));
-    const cudaError_t e = cudaMemcpy(q, sl.data(), sizeof(int4) * sl.size(), cudaMemcpyHostToDevice);
+    // on the context's stream, with which a copy by the default stream has no order (the list is static)
+    const cudaError_t e = cudaMemcpyAsync(q, sl.data(), sizeof(int4) * sl.size(), cudaMemcpyHostToDevice, ctx->stream);
     if (e != cudaSuccess) cudaFree(q);
     CUBE_CUDA_TRY(ctx, e);
     ctx->halo_shells = q;

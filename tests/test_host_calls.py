@@ -58,3 +58,19 @@ s.a, s.sigma_vi, s.mass_p_cdm, s.vsim2phys = 0.5, 0.01, 1.0, 1.0
 halos, members, hid, npeak = g.halofind(s, hid_len=10)
 print(json.dumps([len(halos), len(members), hid.tolist(), npeak]))
 """) == [0, 0, [0] * 10, 0]
+
+
+def test_halofind_orders_everything_on_the_context_stream(child):
+    """A copy by the default stream is not ordered with the context's own: the kernels of the
+    first call could read the list of shells before it is there."""
+    log = child("""
+g = empty_box()
+fake.fake_clear()
+s = CubeScalars()
+s.a, s.sigma_vi, s.mass_p_cdm, s.vsim2phys = 0.5, 0.01, 1.0, 1.0
+g.halofind(s)
+print(json.dumps(calls()))
+""")
+    assert [c for c in log if c["call"] == "launch"] and [c for c in log if c["name"] == "h2d"]
+    streams = {c["stream"] for c in log}
+    assert len(streams) == 1 and streams != {"(nil)"}, [c for c in log if c["stream"] == "(nil)"]
