@@ -373,14 +373,24 @@ int32_t cube_load_state(cube_ctx* ctx, int64_t nplocal, const void* xp, const vo
     ctx->err = "nplocal exceeds the context capacity";
     return CUBE_ERR_CAPACITY;
   }
-  // Into the second buffers (the arrays as they come in scratch of the re-bin), checked
-  // by the scan's total and swapped in at the end: a state whose counts do not add up
-  // leaves the resident one as it is.  (Adding the counts on the host first kept the
-  // copies waiting: 7 ms for the 256^3 cells of a box of 512^3 particles.)
+  // Into the second buffers (the arrays as they come in scratch of the re-bin), swapped in
+  // at the end: a refused or failed load leaves the resident state as it is.  The counts come
+  // first, and only if their total is nplocal are arrays of that length read from the host.
+  // (The total is the scan's: adding the counts on the host kept the copies waiting 7 ms
+  // for the 256^3 cells of a box of 512^3 particles; the wait for their own copy is 1.2 ms.)
   const int64_t nce = ctx->ncells;
   const size_t np = (size_t)nplocal;
   cudaStream_t st = ctx->stream;
   CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), st));
+  CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->rhoc2, rhoc, 4 * (size_t)nce, cudaMemcpyHostToDevice, st));
+  const int src = cube_exclusive_scan(ctx, ctx->rhoc2, nce, ctx->cell_start2, &ctx->dscal->np_new);
+  const cudaError_t counted = cube_read_dscal(ctx);
+  if (src) return src;
+  CUBE_CUDA_TRY(ctx, counted);
+  if (ctx->hscal->np_new != nplocal) {
+    ctx->err = "sum(rhoc) != nplocal";
+    return CUBE_ERR_PARAM;
+  }
   auto codes = [&](const void* host, void* stage, void* soa, int izip) -> int {
     CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(stage, host, 3 * np * izip, cudaMemcpyHostToDevice, st));
     if (izip == 1) k_aos_to_soa<int8_t><<<1184, 256, 0, st>>>((int8_t*)stage, (int8_t*)soa, nplocal, ctx->cap);
@@ -390,8 +400,6 @@ int32_t cube_load_state(cube_ctx* ctx, int64_t nplocal, const void* xp, const vo
   };
   auto copy = [&]() -> int {
     int rc;
-    CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->rhoc2, rhoc, 4 * (size_t)nce, cudaMemcpyHostToDevice, st));
-    if ((rc = cube_exclusive_scan(ctx, ctx->rhoc2, nce, ctx->cell_start2, &ctx->dscal->np_new))) return rc;
     if ((rc = codes(xp, ctx->slot_r2, ctx->xp2, ctx->izipx))) return rc;  // 8 bytes per particle of scratch each
     if ((rc = codes(vp, ctx->slot_s2, ctx->vp2, ctx->izipv))) return rc;
     if (pid) CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->pid2, pid, 4 * np, cudaMemcpyHostToDevice, st));
@@ -401,13 +409,9 @@ int32_t cube_load_state(cube_ctx* ctx, int64_t nplocal, const void* xp, const vo
     return CUBE_OK;
   };
   const int rc = copy();
-  const cudaError_t done = cube_read_dscal(ctx);  // the host's arrays are free again
+  const cudaError_t done = cudaStreamSynchronize(st);  // the host's arrays are free again
   if (rc) return rc;
   CUBE_CUDA_TRY(ctx, done);
-  if (ctx->hscal->np_new != nplocal) {
-    ctx->err = "sum(rhoc) != nplocal";
-    return CUBE_ERR_PARAM;
-  }
   std::swap(ctx->xp, ctx->xp2);
   std::swap(ctx->vp, ctx->vp2);
   if (pid) std::swap(ctx->pid, ctx->pid2);

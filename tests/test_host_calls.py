@@ -74,3 +74,24 @@ print(json.dumps(calls()))
     assert [c for c in log if c["call"] == "launch"] and [c for c in log if c["name"] == "h2d"]
     streams = {c["stream"] for c in log}
     assert len(streams) == 1 and streams != {"(nil)"}, [c for c in log if c["stream"] == "(nil)"]
+
+
+def test_contradicting_counts_are_refused_before_the_particle_arrays_are_read(child):
+    """A caller whose particle count is larger than its arrays (the kernels do nothing here: the
+    device's total stays 0 against 64)."""
+    code, read, log = child("""
+g = empty_box()
+xp, vp, pid = np.zeros((64, 3), np.int16), np.zeros((64, 3), np.int16), np.zeros(64, np.int32)
+rhoc, vf = np.zeros(16 ** 3, np.int32), np.zeros((16 ** 3, 3), np.float32)
+fake.fake_clear()
+try:
+    g.load_state(xp, vp, pid, rhoc, vf)
+    code = 0
+except CubeError as e:
+    code = e.code
+read = [c["src"] == hex(a.ctypes.data) for a in (xp, vp, pid, vf, rhoc) for c in calls() if c["name"] == "h2d"]
+n = sum(c["name"] == "h2d" for c in calls())
+print(json.dumps([code, [any(read[i * n:(i + 1) * n]) for i in range(5)], calls()]))
+""")
+    assert code == 1
+    assert read == [False] * 4 + [True], log
