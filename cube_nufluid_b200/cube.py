@@ -163,6 +163,11 @@ class Cube:
         pid = None if pid is None else np.ascontiguousarray(pid, dtype=np.int32)
         rhoc = np.ascontiguousarray(rhoc, dtype=np.int32)
         vfield = np.ascontiguousarray(vfield, dtype=np.float32)
+        n, nce = xp.shape[0], self.nc ** 3  # the library reads this much of each array
+        for name, a, need in (("xp", xp, 3 * n * self.p.izipx), ("vp", vp, 3 * n * self.p.izipv), ("pid", pid, 4 * n),
+                              ("rhoc", rhoc, 4 * nce), ("vfield", vfield, 12 * nce)):
+            if a is not None and a.nbytes < need:
+                raise CubeError(1, f"{name} is shorter than a state of {n} particles in {nce} cells")
         self._check(self.L.cube_load_state(self.h, xp.shape[0], _ptr(xp), _ptr(vp), _ptr(pid), _ptr(rhoc),
                                            _ptr(vfield)))
 

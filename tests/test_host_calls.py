@@ -95,3 +95,24 @@ print(json.dumps([code, [any(read[i * n:(i + 1) * n]) for i in range(5)], calls(
 """)
     assert code == 1
     assert read == [False] * 4 + [True], log
+
+
+@pytest.mark.parametrize("short", range(5))
+def test_load_state_refuses_arrays_shorter_than_the_state(child, short):
+    """nplocal is the length of xp: an array with fewer bytes than that state has is refused
+    and none is read; one that is longer is taken as before."""
+    code, copies = child(f"""
+g = Cube(make_params(16, 2, izipx=2, izipv=2), np_capacity=64)
+arrays = [np.zeros((64, 3), np.int16), np.zeros((64, 3), np.int16), np.zeros(64, np.int32),
+          np.zeros(16 ** 3, np.int32), np.zeros((16 ** 3, 3), np.float32)]
+short = {short}
+arrays[short] = arrays[short].astype(np.int8) if short == 0 else arrays[short][:-1]
+fake.fake_clear()
+try:
+    g.load_state(*arrays)
+    code = 0
+except CubeError as e:
+    code = e.code
+print(json.dumps([code, sum(c["name"] == "h2d" for c in calls())]))
+""")
+    assert (code, copies) == (1, 0)
