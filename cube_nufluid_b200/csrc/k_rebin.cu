@@ -828,6 +828,7 @@ int run_rebin_crowded(cube_ctx* ctx, RebinArgs& A) {
   // Cells beyond the block sorter first, on a stream beside the context's: few CTAs whose
   // time is the largest cell's, while the other sorters fill the GPU (four steps of a
   // clustered 128^3 box: 10.7 ms one after the other, 9.3 ms so).
+  int rc = CUBE_OK;
   if (hv[0]) {
     // one slot per SM of keys (mmax, a power of two) and three velocity columns
     // of mmax: the scratch is reallocated only when mmax doubles
@@ -851,15 +852,17 @@ int run_rebin_crowded(cube_ctx* ctx, RebinArgs& A) {
     }
     CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->side_ev[0], ctx->stream));
     CUBE_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->side, ctx->side_ev[0], 0));
-    k_rebin_huge_order<<<1, 1024, 0, ctx->side>>>(A);
-    CUBE_LAUNCH_CHECK(ctx);
-    k_rebin_huge<ZX, ZV><<<grid, 1024, tsmem, ctx->side>>>(
-        A, reinterpret_cast<unsigned long long*>(ctx->rebin_scratch), slot, mmax);
-    CUBE_LAUNCH_CHECK(ctx);
-    CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->side_ev[1], ctx->side));
+    // (an error from here on still waits for the side stream)
+    rc = [&]() -> int {
+      k_rebin_huge_order<<<1, 1024, 0, ctx->side>>>(A);
+      CUBE_LAUNCH_CHECK(ctx);
+      k_rebin_huge<ZX, ZV><<<grid, 1024, tsmem, ctx->side>>>(
+          A, reinterpret_cast<unsigned long long*>(ctx->rebin_scratch), slot, mmax);
+      CUBE_LAUNCH_CHECK(ctx);
+      return CUBE_OK;
+    }();
   }
-  // (an error from here on still waits for the side stream)
-  const int rc0 = [&]() -> int {
+  if (!rc) rc = [&]() -> int {
     if (hv[3]) {
       const size_t wsmem = sizeof(unsigned long long) * 4 * WARP_MAX * WARP_WARPS;
       CUBE_CUDA_TRY(ctx, cube_smem_limit(ctx, k_rebin_warp<ZX, ZV>, wsmem));
@@ -878,11 +881,16 @@ int run_rebin_crowded(cube_ctx* ctx, RebinArgs& A) {
     }
     return CUBE_OK;
   }();
-  if (hv[0]) CUBE_CUDA_TRY(ctx, cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0));
-  if (rc0) return rc0;
+  if (hv[0]) {
+    cudaError_t e = cudaEventRecord(ctx->side_ev[1], ctx->side);
+    if (e == cudaSuccess) e = cudaStreamWaitEvent(ctx->stream, ctx->side_ev[1], 0);
+    if (e != cudaSuccess) cudaStreamSynchronize(ctx->side);
+    CUBE_CUDA_TRY(ctx, e);
+  }
+  if (rc) return rc;
   // their entries, over work items of the new layout
   int64_t ni = 0;
-  const int rc = cube_cell_items(ctx, A.start2, false, &A.items, &ni);
+  rc = cube_cell_items(ctx, A.start2, false, &A.items, &ni);
   if (rc) return rc;
   k_rebin_emit<ZX, ZV><<<(unsigned)ni, 256, 0, ctx->stream>>>(A);
   CUBE_LAUNCH_CHECK(ctx);

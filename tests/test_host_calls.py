@@ -9,6 +9,8 @@ import sys
 
 import pytest
 
+from cube_nufluid_b200.build import ARCH, CSRC, FLAGS, NVCC
+
 TESTS = os.path.dirname(os.path.abspath(__file__))
 ROOT = os.path.dirname(TESTS)
 CUDA = os.environ.get("CUDA_HOME", "/usr/local/cuda")
@@ -116,3 +118,41 @@ except CubeError as e:
 print(json.dumps([code, sum(c["name"] == "h2d" for c in calls())]))
 """)
     assert (code, copies) == (1, 0)
+
+
+def test_refused_launch_on_the_side_stream_still_joins_it(child, tmp_path):
+    """The largest cells are sorted on a stream beside the context's.  When the second of its two
+    launches is refused, the call fails, and the context's stream waits for the first."""
+    names = ["n_huge", "max_huge"]
+    (tmp_path / "o.cu").write_text(
+        '#include "cube_internal.cuh"\n#include <cstdio>\nint main() { printf("%zu ' + "%zu " * len(names) + '", sizeof(DevScal)'
+        + "".join(f", offsetof(DevScal, {n})" for n in names) + "); }\n")
+    subprocess.run([NVCC, *ARCH, *FLAGS, "-I", CSRC, "-I", os.path.join(ROOT, "include"), "-o", str(tmp_path / "o"),
+                    str(tmp_path / "o.cu")], check=True)
+    size, n_huge, max_huge = map(int, subprocess.run([str(tmp_path / "o")], capture_output=True, text=True).stdout.split())
+    code, log = child(f"""
+g = empty_box()
+fake.fake_poke({size}, {n_huge}, 2)
+fake.fake_poke({size}, {max_huge}, 20000)
+fake.fake_refuse(b"k_rebin_hugeI")
+fake.fake_clear()
+s = CubeScalars()
+s.dt = s.dt_old = 1.0
+s.sigma_vi = 0.01
+try:
+    g.update_x(s)
+    code = 0
+except CubeError as e:
+    code = e.code
+print(json.dumps([code, calls()]))
+""")
+    assert code == 3
+    at = next(i for i, c in enumerate(log) if c["call"] == "refused")
+    side = log[at]["stream"]
+    assert log[at - 1]["stream"] == side and "k_rebin_huge_order" in log[at - 1]["name"]
+    main = log[0]["stream"]
+    assert main != side
+    joined = [c for i, c in enumerate(log[at:]) if c["call"] == "cudaStreamWaitEvent" and c["stream"] == main
+              and any(e["call"] == "cudaEventRecord" and e["src"] == c["src"] and e["stream"] == side
+                      for e in log[at:at + i])]
+    assert joined or any(c["call"] == "cudaStreamSynchronize" and c["stream"] == side for c in log[at:])
