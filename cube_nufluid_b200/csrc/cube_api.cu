@@ -85,9 +85,10 @@ int check_device_error(cube_ctx* ctx, bool read = false) {
   return CUBE_OK;
 }
 
-void set_phase(cube_ctx* ctx, int phase, int first, int last) {
-  ctx->phase_ev[phase][0] = (signed char)first;
-  ctx->phase_ev[phase][1] = (signed char)last;
+// the times of a phase of the call, which has finished
+void set_phase(cube_ctx* ctx, EvCall call, int phase, int first, int last) {
+  ctx->phase_ev[phase][0] = ctx->ev[ctx->ev_set[call]][first];
+  ctx->phase_ev[phase][1] = ctx->ev[ctx->ev_set[call]][last];
 }
 
 float uint_as_float(unsigned int u) {
@@ -248,8 +249,9 @@ void cube_destroy(cube_ctx* ctx) {
   for (double* t : ctx->vdec)
     if (t) cudaFree(t);
   if (ctx->hscal) cudaFreeHost(ctx->hscal);
-  for (int i = 0; i < 16; ++i)
-    if (ctx->ev[i]) cudaEventDestroy(ctx->ev[i]);
+  for (auto& set : ctx->ev)
+    for (cudaEvent_t e : set)
+      if (e) cudaEventDestroy(e);
   for (cudaEvent_t e : ctx->side_ev)
     if (e) cudaEventDestroy(e);
   if (ctx->side) cudaStreamDestroy(ctx->side);
@@ -275,8 +277,6 @@ int32_t cube_create(const cube_params* params, int64_t np_capacity, const float*
     return CUBE_ERR_PARAM;
   }
   cube_ctx* ctx = new cube_ctx();
-  memset(ctx->ev, 0, sizeof(ctx->ev));
-  memset(ctx->phase_ev, -1, sizeof(ctx->phase_ev));
   ctx->P = P;
   ctx->nc = P.nc; ctx->nnt = P.nnt; ctx->nt = P.nc / P.nnt; ctx->ncell = P.ncell; ctx->ncb = P.ncb;
   ctx->nte = ctx->nt + 2 * ctx->ncb; ctx->nf = P.nc * P.ncell;
@@ -308,8 +308,9 @@ int32_t cube_create(const cube_params* params, int64_t np_capacity, const float*
     if (cudaDeviceGetAttribute(&ctx->num_sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || ctx->num_sms <= 0)
       ctx->num_sms = 148;
   }
-  for (int i = 0; i < 16; ++i)
-    if (cudaEventCreate(&ctx->ev[i]) != cudaSuccess) { ctx->err = "cudaEventCreate failed"; return fail(CUBE_ERR_CUDA); }
+  for (auto& set : ctx->ev)
+    for (cudaEvent_t& e : set)
+      if (cudaEventCreate(&e) != cudaSuccess) { ctx->err = "cudaEventCreate failed"; return fail(CUBE_ERR_CUDA); }
   const int64_t cap = ctx->cap, nce = ctx->ncells;
   auto A = [&](void** p, size_t bytes) -> bool {
     if (cudaMalloc(p, bytes) != cudaSuccess) {
@@ -456,7 +457,8 @@ int32_t cube_store_state(cube_ctx* ctx, int64_t* nplocal, void* xp, void* vp, in
 int32_t cube_update_x(cube_ctx* ctx, cube_scalars* io) {
   if (!ctx || !io) return CUBE_ERR_PARAM;
   if (!ctx->state_loaded) return CUBE_ERR_STATE;
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0], ctx->stream));
+  cudaEvent_t* ev = ctx->ev[ctx->ev_set[EV_UPDATE_X]];
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[0], ctx->stream));
   CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), ctx->stream));
   int rc = cube_rebin(ctx, io, false);
   if (rc) return rc;
@@ -476,7 +478,7 @@ int32_t cube_update_x(cube_ctx* ctx, cube_scalars* io) {
     if (cube_rebin_has_crowded(ctx) && (rc = cube_rebin(ctx, io, true))) return rc;
   }
   for (;;) {
-    CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[1], ctx->stream));
+    CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[1], ctx->stream));
     if ((rc = cube_stats_sums(ctx, slot_cell, dec, coef))) return rc;
     if ((rc = check_device_error(ctx))) return rc;
     if (sorted || !cube_rebin_has_crowded(ctx)) break;
@@ -504,7 +506,8 @@ int32_t cube_update_x(cube_ctx* ctx, cube_scalars* io) {
   io->std_vsim = sqrt(sums[2] / npg);
   io->sigma_vi_new = (float)(io->std_vsim_res / (double)sqrtf(3.f));
   io->nplocal = ctx->np;
-  set_phase(ctx, 0, 0, 1);
+  set_phase(ctx, EV_UPDATE_X, 0, 0, 1);
+  ctx->ev_set[EV_UPDATE_X] ^= 1;
   return CUBE_OK;
 }
 
@@ -512,27 +515,28 @@ int32_t cube_particle_mesh(cube_ctx* ctx, cube_scalars* io) {
   if (!ctx || !io) return CUBE_ERR_PARAM;
   if (!ctx->state_loaded) return CUBE_ERR_STATE;
   CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), ctx->stream));
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[2], ctx->stream));
+  cudaEvent_t* ev = ctx->ev[ctx->ev_set[EV_PARTICLE_MESH]];
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[2], ctx->stream));
   int rc = cube_deposit(ctx, io);
   if (rc) return rc;
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[3], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[3], ctx->stream));
   const KickScale ks = {io->a_mid, io->dt, ctx->codec.pi_f, 1, 1.0f / 6.0f, 1.0f / ctx->codec.pi_f};
   if ((rc = cube_fft_poisson(ctx, ctx->fine, &ctx->dscal->f2_fine_bits, ks))) return rc;
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[4], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[4], ctx->stream));
   if ((rc = cube_fft_poisson(ctx, ctx->coarse, &ctx->dscal->f2_coarse_bits, ks))) return rc;
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[5], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[5], ctx->stream));
   if ((rc = cube_kick(ctx, io))) return rc;
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[6], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[6], ctx->stream));
   if (ctx->nu.on) {
     if ((rc = cube_nu_gravity(ctx, io))) return rc;
-    CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[9], ctx->stream));
+    CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[9], ctx->stream));
   }
   if (ctx->nu.on && (rc = cube_tree_sums_async(ctx, ctx->nu.partial, ctx->nu.nparts, 0, 1, ctx->dscal->sums))) return rc;
   if ((rc = check_device_error(ctx))) return rc;
   cube_mass_sums(ctx->hscal->mass, io->mass_p_cdm, &io->testrhof, &io->testrhoc);
   if (ctx->nu.on) {
     io->testrhof += ctx->hscal->sums[0];
-    set_phase(ctx, 6, 6, 9);
+    set_phase(ctx, EV_PARTICLE_MESH, 6, 6, 9);
   }
   // the meshes hold force*s; max f^2 in force units
   const double s2 = (double)cube_kick_scalar(ks) * (double)cube_kick_scalar(ks);
@@ -541,7 +545,8 @@ int32_t cube_particle_mesh(cube_ctx* ctx, cube_scalars* io) {
   for (int d = 0; d < 3; ++d) io->vmax[d] = uint_as_float(ctx->hscal->vmax_bits[d]);
   io->sigma_vi = io->sigma_vi_new;  // pm.f90:180
   dt_constraints(ctx, io);
-  for (int ph = 2; ph < 6; ++ph) set_phase(ctx, ph, ph, ph + 1);
+  for (int ph = 2; ph < 6; ++ph) set_phase(ctx, EV_PARTICLE_MESH, ph, ph, ph + 1);
+  ctx->ev_set[EV_PARTICLE_MESH] ^= 1;
   return CUBE_OK;
 }
 
@@ -549,7 +554,7 @@ int32_t cube_ext_pp_force(cube_ctx* ctx, cube_scalars* io) {
   if (!ctx || !io) return CUBE_ERR_PARAM;
   if (!ctx->state_loaded) return CUBE_ERR_STATE;
   CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), ctx->stream));
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[7], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[ctx->ev_set[EV_PP]][7], ctx->stream));
   bool read = false;
   int rc = cube_pp(ctx, io, &read);
   if (rc) return rc;
@@ -561,7 +566,8 @@ int32_t cube_ext_pp_force(cube_ctx* ctx, cube_scalars* io) {
   const float pi_f = ctx->codec.pi_f;
   const float GG = cube_fdiv(cube_fdiv(1.0f, 6.0f), pi_f);
   io->dt_pp = cube_fdiv(cube_fmul(1.0f, sqrtf(1.0f)), cube_fmul(cube_fmul(sqrtf(io->f2_max_pp), io->a_mid), GG));
-  set_phase(ctx, 1, 7, 8);
+  set_phase(ctx, EV_PP, 1, 7, 8);
+  ctx->ev_set[EV_PP] ^= 1;
   if (io->itest1 != ctx->np) {
     ctx->err = "PP did not update every particle once";
     return CUBE_ERR_STATE;
@@ -646,7 +652,8 @@ int32_t cube_nu_evolve(cube_ctx* ctx, float dt, float* dtg, int32_t dir, float a
   }
   NuState& N = ctx->nu;
   if (!(a >= N.ai)) return CUBE_OK;  // dfld_evolve: before the turn-on nothing moves
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[10], ctx->stream));
+  cudaEvent_t* ev = ctx->ev[ctx->ev_set[EV_NU]];
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[10], ctx->stream));
   const unsigned int big = float_as_uint(1e9f);
   const unsigned int init[3] = {big, big, big};
   CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->dscal->nu_dt_bits, init, sizeof(init), cudaMemcpyHostToDevice, ctx->stream));
@@ -655,7 +662,7 @@ int32_t cube_nu_evolve(cube_ctx* ctx, float dt, float* dtg, int32_t dir, float a
     if (rc) return rc;
     if ((rc = cube_nu_timestep(ctx, N.fl[k], &ctx->dscal->nu_dt_bits[k]))) return rc;
   }
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[11], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ev[11], ctx->stream));
   unsigned int bits[3];
   CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(bits, ctx->dscal->nu_dt_bits, sizeof(bits), cudaMemcpyDeviceToHost, ctx->stream));
   CUBE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
@@ -664,7 +671,8 @@ int32_t cube_nu_evolve(cube_ctx* ctx, float dt, float* dtg, int32_t dir, float a
     if (d == 1e9f) d = 1.f;
     *dtg = std::min(*dtg, d);
   }
-  set_phase(ctx, 6, 10, 11);
+  set_phase(ctx, EV_NU, 6, 10, 11);
+  ctx->ev_set[EV_NU] ^= 1;
   return CUBE_OK;
 }
 
@@ -698,13 +706,13 @@ int32_t cube_debug_time_poisson(cube_ctx* ctx, int32_t reps, float* ms) {
   CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), ctx->stream));
   int rc = cube_fft_poisson(ctx, ctx->fine, &ctx->dscal->f2_fine_bits, ks);  // warm-up
   if (rc) return rc;
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[12], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0][12], ctx->stream));
   for (int r = 0; r < reps; ++r)
     if ((rc = cube_fft_poisson(ctx, ctx->fine, &ctx->dscal->f2_fine_bits, ks))) return rc;
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[13], ctx->stream));
-  CUBE_CUDA_TRY(ctx, cudaEventSynchronize(ctx->ev[13]));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[0][13], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventSynchronize(ctx->ev[0][13]));
   float t = 0.f;
-  cudaEventElapsedTime(&t, ctx->ev[12], ctx->ev[13]);
+  cudaEventElapsedTime(&t, ctx->ev[0][12], ctx->ev[0][13]);
   *ms = t / (float)reps;
   return CUBE_OK;
 }
@@ -782,10 +790,10 @@ int32_t cube_phase_times(cube_ctx* ctx, float* ms8) {
   if (!ctx || !ms8) return CUBE_ERR_PARAM;
   float tot = 0;
   for (int i = 0; i < 7; ++i) {
-    const signed char* e = ctx->phase_ev[i];
+    const cudaEvent_t* e = ctx->phase_ev[i];
     ms8[i] = 0.f;
-    if (e[0] >= 0 && cudaEventElapsedTime(&ms8[i], ctx->ev[e[0]], ctx->ev[e[1]]) != cudaSuccess) {
-      cudaGetLastError();  // a phase whose call was not finished has no time
+    if (e[0] && cudaEventElapsedTime(&ms8[i], e[0], e[1]) != cudaSuccess) {
+      cudaGetLastError();
       ms8[i] = 0.f;
     }
     tot += ms8[i];

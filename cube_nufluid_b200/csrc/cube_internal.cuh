@@ -119,6 +119,9 @@ struct NuState {
   int nparts = 0;
 };
 
+// the calls that are timed (cube_phase_times)
+enum EvCall { EV_UPDATE_X, EV_PP, EV_PARTICLE_MESH, EV_NU };
+
 struct cube_ctx {
   cube_params P;
   int nc, nnt, nt, ncell, ncb, nte, nf, nvbin;
@@ -173,8 +176,11 @@ struct cube_ctx {
   DevScal* hscal;                 // pinned host mirror
   float2* sbuf;                   // spare spectrum buffer for the forward z pass
   // timing
-  cudaEvent_t ev[16];
-  signed char phase_ev[8][2];  // first and last event of each phase of the last calls (first < 0: none yet)
+  // events of the calls that are timed, twice: a call records into the set that its last
+  // finished one did not use, so that one which fails leaves the times that are there
+  cudaEvent_t ev[2][16] = {};
+  int ev_set[4] = {0, 0, 0, 0};     // the set that each call (EvCall) records into next
+  cudaEvent_t phase_ev[8][2] = {};  // first and last event of each phase of the last finished calls
   std::vector<const void*> smem_raised;  // kernels whose dynamic shared-memory limit this context has raised
   long long launches;
   std::string err;

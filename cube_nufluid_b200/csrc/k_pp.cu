@@ -1279,7 +1279,7 @@ int launch_pp(cube_ctx* ctx, const cube_scalars* io, bool* read) {
   CUBE_LAUNCH_CHECK(ctx);
   k_pp_crowd_list<<<(unsigned)((nbricks + 255) / 256), 256, 0, ctx->stream>>>(Q, nbricks);
   CUBE_LAUNCH_CHECK(ctx);
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[8], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[ctx->ev_set[EV_PP]][8], ctx->stream));
   CUBE_CUDA_TRY(ctx, cube_read_dscal(ctx));
   const unsigned long long ndense = ctx->hscal->pp_dense;
   *read = true;
@@ -1293,7 +1293,7 @@ int launch_pp(cube_ctx* ctx, const cube_scalars* io, bool* read) {
   kb<<<(unsigned)ndense, PP_THREADS, smem, ctx->stream>>>(ctx->xp, ctx->vp, ctx->cell_start, ctx->nc, ctx->nt,
                                                           ctx->nnt, A, spill, ctx->dscal, Q.dense_list);
   CUBE_LAUNCH_CHECK(ctx);
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[8], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[ctx->ev_set[EV_PP]][8], ctx->stream));
   CUBE_CUDA_TRY(ctx, cube_read_dscal(ctx));
   const unsigned long long nspill = ctx->hscal->n_big;
   if (!nspill) return CUBE_OK;
@@ -1345,7 +1345,7 @@ int launch_pp(cube_ctx* ctx, const cube_scalars* io, bool* read) {
   CUBE_LAUNCH_CHECK(ctx);
   k_pp_crowd<ZX, ZV><<<(unsigned)chunks, PP_THREADS, 0, ctx->stream>>>(ctx->vp, A, C, ctx->dscal);
   CUBE_LAUNCH_CHECK(ctx);
-  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[8], ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaEventRecord(ctx->ev[ctx->ev_set[EV_PP]][8], ctx->stream));
   // the host copy of meta must outlive the asynchronous upload
   CUBE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
   return CUBE_OK;

@@ -14,12 +14,13 @@ static std::string g_log, g_refused;
 static std::map<const void*, std::string> g_names;
 static size_t g_poke_size = 0;
 static std::vector<std::pair<size_t, unsigned long long>> g_pokes;
-static long g_handles = 0;
+static long g_handles = 0, g_calls = 0;
 
 static void note(const char* what, const std::string& name, const void* src, cudaStream_t st) {
   char b[96];
   snprintf(b, sizeof(b), " %p %p\n", src, (void*)st);
   g_log += std::string(what) + " " + name + b;
+  ++g_calls;
 }
 
 extern "C" {
@@ -92,9 +93,15 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t e, unsigned) { note(
 cudaError_t cudaEventCreate(cudaEvent_t* e) { *e = (cudaEvent_t)++g_handles; return cudaSuccess; }
 cudaError_t cudaEventCreateWithFlags(cudaEvent_t* e, unsigned) { return cudaEventCreate(e); }
 cudaError_t cudaEventDestroy(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) { note("cudaEventRecord", "-", e, s); return cudaSuccess; }
+// an event's time is the number of calls before it
+static std::map<cudaEvent_t, long> g_time;
+cudaError_t cudaEventRecord(cudaEvent_t e, cudaStream_t s) {
+  note("cudaEventRecord", "-", e, s);
+  g_time[e] = g_calls;
+  return cudaSuccess;
+}
 cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t, cudaEvent_t) { *ms = 1.f; return cudaSuccess; }
+cudaError_t cudaEventElapsedTime(float* ms, cudaEvent_t a, cudaEvent_t b) { *ms = g_time[b] - g_time[a]; return cudaSuccess; }
 cudaError_t cudaGetDevice(int* d) { *d = 0; return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute(int* v, cudaDeviceAttr a, int) {
   *v = a == cudaDevAttrMultiProcessorCount ? 148 : 232448;

@@ -156,3 +156,32 @@ print(json.dumps([code, calls()]))
               and any(e["call"] == "cudaEventRecord" and e["src"] == c["src"] and e["stream"] == side
                       for e in log[at:at + i])]
     assert joined or any(c["call"] == "cudaStreamSynchronize" and c["stream"] == side for c in log[at:])
+
+
+def test_phase_times_are_those_of_the_last_finished_call(child):
+    """A call that fails on its way leaves the times that are there (event times here: calls)."""
+    before, after, again = child("""
+g = empty_box()
+s = CubeScalars()
+s.dt = s.dt_old = 1.0
+s.a = s.a_mid = 0.5
+s.sigma_vi = s.sigma_vi_new = 0.01
+g.update_x(s)
+g.particle_mesh(s)
+before = g.phase_times()
+for kernel, call in ((b"k_rebin_count", g.update_x), (b"k_coarse_finalize", g.particle_mesh)):
+    fake.fake_refuse(kernel)
+    try:
+        call(s)
+        raise SystemExit("not refused")
+    except CubeError as e:
+        assert e.code == 3
+after = g.phase_times()
+fake.fake_refuse(b"")
+g.update_x(s)
+g.particle_mesh(s)
+print(json.dumps([before, after, g.phase_times()]))
+""")
+    assert [t > 0 for t in before] == [True, False, True, True, True, True, False, True]
+    assert after == before
+    assert [t > 0 for t in again] == [t > 0 for t in before]
