@@ -389,16 +389,18 @@ __device__ __forceinline__ float cube_kick_scale(float f, const KickScale& k) {
 // to q = Q atan(x), x = coef v, Q = nvbin_m1/pi_f, so FP32 arithmetic decides it unless
 // q lies close to k + 1/2.  x is split off the nearest of the VENC_N breakpoints c_j
 // (32 per octave from 2^-7 to 2^9, found from the bits of the FP32 x; c_0 = 0 below
-// 2^-7): atan(x) = atan(c_j) + atan(u), u = (x - c_j)/(1 + x c_j), |u| < 0.0079, and
-// Q atan(c_j) is tabulated as an integer plus an FP32 rest.  The difference x - c_j is
-// formed in FP64 (c_j has seven significant bits, so the high word of its double is
-// all of it) and rounded once; with the roundings of the denominator, the approximate
-// quotient (2 ulp), the polynomial (the dropped u^5/5 is 3e-12) and the final
-// multiply-add, Q atan(u), at most 83 in magnitude, is off by less than 1e-4.  The
-// integer is accepted unless the fraction comes within VENC_BAND = 2e-4 of 1/2 (one
-// encode in 2500), where the exact FP64 evaluation decides, as it does beyond 2^9 and
-// for NaN.  (An FP64 evaluation from 64 angle breakpoints with a 1e-9 band, the form
-// before, took 83 warp instructions per encode and six conversions; this takes 30.)
+// 2^-7): atan(x) = atan(c_j) + atan(u), u = (x - c_j)/(1 + x c_j), |u| <= 2^-7 (just below 2^-7,
+// where c_0 = 0, and nearly so above 1), and Q atan(c_j) is tabulated as an integer plus an FP32
+// rest.  The difference x - c_j is formed in FP64 (c_j has seven significant bits, so the
+// high word of its double is all of it) and rounded once.  Q atan(u) reaches 163 in magnitude.
+// Its relative error, in units of 2^-24: 1 from the difference, 2 from the denominator, 4 from
+// the approximate quotient (2 ulp), 1.5 from the polynomial, 1 from Q; in all 9.3e-5 at 163, and
+// 8e-6 from the final multiply-add and 2e-7 from the dropped u^5/5 (at most 6e-12) beside it: at
+// most 1.02e-4 where everything falls together.  The integer is accepted unless the fraction comes
+// within VENC_BAND = 2e-4 of 1/2, twice that (one encode in 2500), where the exact FP64
+// evaluation decides, as it does beyond 2^9 and for NaN.  (An FP64 evaluation from 64 angle
+// breakpoints with a 1e-9 band, the form before, took 83 warp instructions per encode and six
+// conversions; this takes 30.)
 constexpr int VENC_LO = 120, VENC_OCT = 16;        // first octave 2^(120-127), octaves
 constexpr int VENC_N = VENC_OCT * 32 + 1;
 constexpr float VENC_BAND = 2e-4f;

@@ -455,31 +455,35 @@ const double* cube_vdec_table(cube_ctx* ctx, double coef, int* rc) {
 }
 
 namespace {
-// velocities spread over the code range: v = tan(pi*(code + off)/(nvbin-1))/coef with
-// off in (-1, 1) drawn from a hash of the index, so that many land near the
-// rounding boundaries code +- 1/2 (within 1.3e-8 of a boundary, and within 3.3e-4, which
-// covers the fallback's band of 2e-4 in q); the step's encode against cube_vencode
+// velocities spread over the code range: v = tan(pi_f*(code + off)/(nvbin-1))/coef with an
+// integer code, so that the encode's q is code + off, and off of a hash of the index: within
+// 1.3e-8 of the rounding boundary code + 1/2, within 1e-3 of it (both sides of the edges of the
+// FP32 form's band of 2e-4), or anywhere; the step's encode against cube_vencode.
+// seen: mismatches, inputs inside the band, inputs beside it
 __global__ void k_encode_check(cube_codec codec, VencTab tab, double coef, int64_t n, uint64_t seed,
-                               unsigned long long* __restrict__ bad) {
-  unsigned long long nb = 0;
+                               unsigned long long* __restrict__ seen) {
+  unsigned long long bad = 0, inside = 0, beside = 0;
+  const double nb1 = (double)codec.nvbin_m1_f, pif = (double)codec.pi_f;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     uint64_t h = (uint64_t)i * 0x9E3779B97F4A7C15ull + seed;
     h ^= h >> 31; h *= 0xBF58476D1CE4E5B9ull; h ^= h >> 27; h *= 0x94D049BB133111EBull; h ^= h >> 31;
-    const double u = (double)(h >> 11) * 0x1p-53;                        // [0,1)
-    const double half = 0.5 * (double)codec.nvbin_m1_f;
-    const double code = floor(u * (double)codec.nvbin_m1_f) - half;       // whole code range
+    const double u = (double)(h >> 19) * 0x1p-45;                     // [0,1), of other bits than cls and off
+    const double code = floor(u * (nb1 + 1.0)) - 0.5 * (nb1 + 1.0);   // every code
     const int cls = (int)(h & 7);
-    const double off = cls < 3 ? ((double)((h >> 3) & 0xFF) - 128.0) * 1e-10 + 0.5       // near x.5
-                     : cls < 5 ? ((double)((h >> 3) & 0xFFFF) - 32768.0) * 1e-8 + 0.5     // across the
-                                                                                          // FP32 form's band
-                               : ((double)((h >> 3) & 0xFFFF) / 65536.0 - 0.5);          // anywhere
-    const double ang = 3.141592653589793 * (code + off) / (double)codec.nvbin_m1_f;
+    const double off = cls < 3 ? ((double)((h >> 3) & 0xFF) - 128.0) * 1e-10 + 0.5
+                     : cls < 6 ? ((double)((h >> 3) & 0xFFFF) - 32768.0) * 3e-8 + 0.5
+                               : ((double)((h >> 3) & 0xFFFF) / 65536.0 - 0.5);
+    const double ang = pif * (code + off) / nb1;
     if (fabs(ang) >= 1.5707963) continue;
     const double v = tan(ang) / coef;
-    const int32_t ex = cube_vencode(&codec, v, coef);
-    nb += cube_vencode_step(&codec, tab, v, coef) != ex;
+    const double q = nb1 * atan(coef * v) / pif, d = fabs(q - floor(q) - 0.5);
+    inside += d < (double)VENC_BAND;
+    beside += d >= (double)VENC_BAND && d < 1e-3;
+    bad += cube_vencode_step(&codec, tab, v, coef) != cube_vencode(&codec, v, coef);
   }
-  if (nb) atomicAdd(bad, nb);
+  if (bad) atomicAdd(seen, bad);
+  atomicAdd(seen + 1, inside);
+  atomicAdd(seen + 2, beside);
 }
 }  // namespace
 
@@ -545,15 +549,20 @@ int32_t cube_debug_division_check(cube_ctx* ctx, int64_t n, uint64_t seed, int64
 
 int32_t cube_debug_encode_check(cube_ctx* ctx, int64_t n, uint64_t seed, float sigma, int64_t* mismatches) {
   if (!ctx || !mismatches || n < 0) return CUBE_ERR_PARAM;
-  unsigned long long* bad = reinterpret_cast<unsigned long long*>(ctx->red_tmp);
-  CUBE_CUDA_TRY(ctx, cudaMemsetAsync(bad, 0, 8, ctx->stream));
+  unsigned long long* seen = reinterpret_cast<unsigned long long*>(ctx->red_tmp);
+  unsigned long long h[3] = {0, 0, 0};
+  CUBE_CUDA_TRY(ctx, cudaMemsetAsync(seen, 0, sizeof(h), ctx->stream));
   const double coef = cube_vcoef(&ctx->codec, sigma);
-  k_encode_check<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(ctx->codec, cube_venc_tab(ctx), coef, n,
-                                                            seed, bad);
+  k_encode_check<<<ctx->num_sms * 8, 256, 0, ctx->stream>>>(ctx->codec, cube_venc_tab(ctx), coef, n, seed, seen);
   CUBE_LAUNCH_CHECK(ctx);
-  unsigned long long h = 0;
-  CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(&h, bad, 8, cudaMemcpyDeviceToHost, ctx->stream));
+  CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(h, seen, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream));
   CUBE_CUDA_TRY(ctx, cudaStreamSynchronize(ctx->stream));
-  *mismatches = (int64_t)h;
+  *mismatches = (int64_t)h[0];
+  // 3/8 and a fifth of another 3/8 of the inputs lie inside the band, the rest of those beside it
+  if (n >= 4096 && (h[1] < (unsigned long long)n / 4 || h[2] < (unsigned long long)n / 8)) {
+    ctx->err = "encode check: " + std::to_string(h[1]) + " inputs inside the band and " + std::to_string(h[2]) +
+               " beside it of " + std::to_string(n);
+    return CUBE_ERR_STATE;
+  }
   return CUBE_OK;
 }

@@ -343,9 +343,12 @@ int32_t cube_debug_kick_with_force(cube_ctx* ctx, cube_scalars* io, const float*
                                    const float* coarse_force);
 
 /* Compares, for n velocities spread over every code and concentrated at the
- * rounding boundaries, the step's velocity encode (breakpoints and an FP32
- * first guess, falling back to the exact encode near ties) with the exact FP64
- * encode under sigma; *mismatches counts the disagreements (0 expected). */
+ * rounding boundaries, the step's velocity encode (an FP32 evaluation from
+ * breakpoints, the exact encode where that comes near a tie) with the exact FP64
+ * encode under sigma; *mismatches counts the disagreements (0 expected).
+ * CUBE_ERR_STATE if (of 4096 velocities or more) too few came to lie inside the
+ * band in which the exact encode decides, or close beside it, for the check to mean
+ * anything. */
 int32_t cube_debug_encode_check(cube_ctx* ctx, int64_t n, uint64_t seed, float sigma, int64_t* mismatches);
 
 /* Compares, for n quotients shaped like the PP pair term (separation components on
