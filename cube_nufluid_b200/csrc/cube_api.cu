@@ -74,6 +74,32 @@ int alloc_level(cube_ctx* ctx, MeshLevel& L, int n, int fp64) {
   return cube_fft_plan(ctx, L.plan, n);
 }
 
+void free_level(MeshLevel& L) {
+  for (void* q : {(void*)L.rho, (void*)L.force, (void*)L.ext, (void*)L.kern, (void*)L.kernd, (void*)L.plan.tw,
+                  (void*)L.plan.tw2, (void*)L.plan.twd})
+    if (q) cudaFree(q);
+}
+
+// n values in [-1, 1) of a hash
+__global__ void k_noise(float* __restrict__ out, int64_t n, uint64_t seed) {
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    uint64_t h = ((uint64_t)i + 1) * 0x9E3779B97F4A7C15ull ^ seed * 0xD1B54A32D192ED03ull;
+    h ^= h >> 32; h *= 0xBF58476D1CE4E5B9ull; h ^= h >> 29;
+    out[i] = (float)((int64_t)(h >> 40) - (1 << 23)) * 0x1p-23f;
+  }
+}
+
+// words of the first w of each row (pitch rp) that differ
+__global__ void k_row_diff(const uint32_t* __restrict__ a, const uint32_t* __restrict__ b, int64_t rows, int w, int rp,
+                           unsigned long long* __restrict__ bad) {
+  unsigned long long nb = 0;
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < rows * w; i += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t q = i / w * rp + i % w;
+    nb += a[q] != b[q];
+  }
+  if (nb) atomicAdd(bad, nb);
+}
+
 // the device scalars into hscal (unless they are there) and the error they hold
 int check_device_error(cube_ctx* ctx, bool read = false) {
   if (!read) CUBE_CUDA_TRY(ctx, cube_read_dscal(ctx));
@@ -837,6 +863,58 @@ int64_t cube_debug_fetch(cube_ctx* ctx, int32_t which, void* host, int64_t capac
   const cudaError_t e = cudaMemcpy(host, tmp, es * n, cudaMemcpyDeviceToHost);
   cudaFree(tmp);
   return e == cudaSuccess ? n : -1;
+}
+
+int32_t cube_debug_mesh_check(cube_ctx* ctx, int32_t n, uint64_t seed, int64_t* mismatches) {
+  if (!ctx || !mismatches || !cube_fftm_ops(n)) return CUBE_ERR_PARAM;
+  MeshLevel L = {};
+  float *force = nullptr, *spec = nullptr;  // of the general passes
+  const int stockham_only = ctx->P.stockham_only;
+  auto run = [&]() -> int {
+    int rc = alloc_level(ctx, L, n, 0);
+    if (rc) return rc;
+    const size_t vol = (size_t)n * L.plane, nk = (size_t)3 * L.kern_pitch * L.kern_pitch * L.kern_pitch;
+    CUBE_CUDA_TRY(ctx, cudaMalloc(&force, 12 * vol));
+    CUBE_CUDA_TRY(ctx, cudaMalloc(&spec, 4 * vol));
+    CUBE_CUDA_TRY(ctx, cudaDeviceSynchronize());  // the level is cleared on the default stream
+    CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), ctx->stream));
+    const KickScale ks = {0.5f, 0.75f, ctx->codec.pi_f, 1, 1.0f / 6.0f, 1.0f / ctx->codec.pi_f};
+    k_noise<<<1184, 256, 0, ctx->stream>>>(L.kern, (int64_t)nk, seed + 1);
+    CUBE_LAUNCH_CHECK(ctx);
+    unsigned long long* bad = reinterpret_cast<unsigned long long*>(ctx->red_tmp);
+    CUBE_CUDA_TRY(ctx, cudaMemsetAsync(bad, 0, 8, ctx->stream));
+    for (int fixed = 0; fixed < 2; ++fixed) {
+      ctx->P.stockham_only = !fixed;
+      k_noise<<<1184, 256, 0, ctx->stream>>>(L.rho, (int64_t)vol, seed);
+      CUBE_LAUNCH_CHECK(ctx);
+      if ((rc = cube_fft_poisson(ctx, L, fixed ? &ctx->dscal->f2_coarse_bits : &ctx->dscal->f2_fine_bits, ks))) return rc;
+      k_noise<<<1184, 256, 0, ctx->stream>>>(L.rho, (int64_t)vol, seed);
+      CUBE_LAUNCH_CHECK(ctx);
+      int kx_major = 0;
+      if ((rc = cube_fft_forward3(ctx, L, L.rho, &kx_major))) return rc;
+      if (!fixed) {
+        CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(force, L.force, 12 * vol, cudaMemcpyDeviceToDevice, ctx->stream));
+        CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(spec, L.rho, 4 * vol, cudaMemcpyDeviceToDevice, ctx->stream));
+      }
+    }
+    const int64_t rows = (int64_t)n * n;
+    k_row_diff<<<1184, 256, 0, ctx->stream>>>((uint32_t*)L.force, (uint32_t*)force, 3 * rows, n, L.rp, bad);
+    CUBE_LAUNCH_CHECK(ctx);
+    k_row_diff<<<1184, 256, 0, ctx->stream>>>((uint32_t*)L.rho, (uint32_t*)spec, rows, n + 2, L.rp, bad);
+    CUBE_LAUNCH_CHECK(ctx);
+    unsigned long long h = 0;
+    CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(&h, bad, 8, cudaMemcpyDeviceToHost, ctx->stream));
+    CUBE_CUDA_TRY(ctx, cube_read_dscal(ctx));
+    *mismatches = (int64_t)h + (ctx->hscal->f2_fine_bits != ctx->hscal->f2_coarse_bits || !ctx->hscal->f2_fine_bits);
+    return CUBE_OK;
+  };
+  const int rc = run();
+  ctx->P.stockham_only = stockham_only;
+  cudaStreamSynchronize(ctx->stream);
+  free_level(L);
+  cudaFree(force);
+  cudaFree(spec);
+  return rc;
 }
 
 int32_t cube_debug_deposit(cube_ctx* ctx, cube_scalars* io) {

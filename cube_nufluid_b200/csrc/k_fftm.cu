@@ -1,8 +1,9 @@
 /*
  * k_fftm.cu -- launchers of the compile-time mixed-radix mesh passes (k_fftm.cuh).
  *
- * Sizes: every multiple of 8 up to 640 with no prime factor above 5 that the register
- * rows of k_fftr.cu do not cover.  These are all the mesh sizes a box of up to 160
+ * Sizes: the multiples of 8 up to 640 with no prime factor above 5 that the register
+ * rows of k_fftr.cu do not cover, but for 600 (a coarse mesh of it has a fine mesh of
+ * 2400^3 nodes, beyond one GPU).  These are all the other mesh sizes that a box of up to 160
  * coarse cells per side has (its coarse mesh of 8 m cells and its fine mesh of four
  * times that), and larger boxes' coarse meshes.  Other sizes, the FP64 Poisson mode
  * and the stockham_only switch take the passes of k_fft.cu.

@@ -76,6 +76,8 @@ def load_library():
     L.cube_debug_encode_check.restype = C.c_int32
     L.cube_debug_division_check.argtypes = [vp, C.c_int64, C.c_uint64, C.POINTER(C.c_int64)]
     L.cube_debug_division_check.restype = C.c_int32
+    L.cube_debug_mesh_check.argtypes = [vp, C.c_int32, C.c_uint64, C.POINTER(C.c_int64)]
+    L.cube_debug_mesh_check.restype = C.c_int32
     L.cube_make_ic.argtypes = [vp, C.POINTER(CubeIcParams), S]
     L.cube_make_ic.restype = C.c_int32
     L.cube_halofind.argtypes = [vp, S, C.POINTER(CubeHaloArgs), C.POINTER(CubeHaloResult)]
@@ -233,6 +235,12 @@ class Cube:
         """Quotients where the shared-reciprocal division differs from IEEE division."""
         bad = C.c_int64(0)
         self._check(self.L.cube_debug_division_check(self.h, int(n), int(seed), C.byref(bad)))
+        return int(bad.value)
+
+    def debug_mesh_check(self, n: int, seed: int) -> int:
+        """Mesh words where the passes compiled for n per side differ from the general ones."""
+        bad = C.c_int64(0)
+        self._check(self.L.cube_debug_mesh_check(self.h, int(n), int(seed), C.byref(bad)))
         return int(bad.value)
 
     def make_ic(self, ic: dict, seed: int, *, f_cdm: float = 1.0) -> CubeScalars:

@@ -358,6 +358,12 @@ int32_t cube_debug_encode_check(cube_ctx* ctx, int64_t n, uint64_t seed, float s
  * quotients that differ in any bit (0 expected). */
 int32_t cube_debug_division_check(cube_ctx* ctx, int64_t n, uint64_t seed, int64_t* mismatches);
 
+/* Compares, on a mesh of n per side filled with noise (n one of the sizes that have
+ * passes compiled for them, CUBE_ERR_PARAM otherwise), those passes with the general
+ * ones: *mismatches counts the words of the Poisson solve's forces and of the
+ * forward spectrum that differ, and one for another max f^2 (0 expected). */
+int32_t cube_debug_mesh_check(cube_ctx* ctx, int32_t n, uint64_t seed, int64_t* mismatches);
+
 /* Device time of the fine-mesh Poisson solve (FFT passes + Green multiply) on
  * whatever the fine density array holds, averaged over reps runs, in *ms. */
 int32_t cube_debug_time_poisson(cube_ctx* ctx, int32_t reps, float* ms);
