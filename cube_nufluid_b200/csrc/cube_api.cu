@@ -403,18 +403,30 @@ int32_t cube_load_state(cube_ctx* ctx, int64_t nplocal, const void* xp, const vo
   // Into the second buffers (the arrays as they come in scratch of the re-bin), swapped in
   // at the end: a refused or failed load leaves the resident state as it is.  The counts come
   // first, and only if their total is nplocal are arrays of that length read from the host.
-  // (The total is the scan's: adding the counts on the host kept the copies waiting 7 ms
-  // for the 256^3 cells of a box of 512^3 particles; the wait for their own copy is 1.2 ms.)
+  // Up to 2^14 cells the host adds them; beyond, the total is the scan's, read back.  (A call of
+  // eight steps on 16^3 cells: 1.775 ms so, 14 us more with the wait; on 32^3 cells 2.529 ms
+  // with the wait, 8 us more with the sum; the sum of the 256^3 cells of a box of 512^3
+  // particles keeps its copies waiting for 7 ms.)
   const int64_t nce = ctx->ncells;
   const size_t np = (size_t)nplocal;
   cudaStream_t st = ctx->stream;
-  CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), st));
-  CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->rhoc2, rhoc, 4 * (size_t)nce, cudaMemcpyHostToDevice, st));
-  const int src = cube_exclusive_scan(ctx, ctx->rhoc2, nce, ctx->cell_start2, &ctx->dscal->np_new);
-  const cudaError_t counted = cube_read_dscal(ctx);
-  if (src) return src;
-  CUBE_CUDA_TRY(ctx, counted);
-  if (ctx->hscal->np_new != nplocal) {
+  auto counts = [&](long long* sum) -> int {
+    CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->rhoc2, rhoc, 4 * (size_t)nce, cudaMemcpyHostToDevice, st));
+    return cube_exclusive_scan(ctx, ctx->rhoc2, nce, ctx->cell_start2, sum);
+  };
+  const bool add_here = nce <= (1 << 14);
+  int64_t total = 0;
+  if (add_here) {
+    for (int64_t c = 0; c < nce; ++c) total += rhoc[c];
+  } else {
+    CUBE_CUDA_TRY(ctx, cudaMemsetAsync(ctx->dscal, 0, sizeof(DevScal), st));
+    const int rc = counts(&ctx->dscal->np_new);
+    const cudaError_t done = cube_read_dscal(ctx);
+    if (rc) return rc;
+    CUBE_CUDA_TRY(ctx, done);
+    total = ctx->hscal->np_new;
+  }
+  if (total != nplocal) {
     ctx->err = "sum(rhoc) != nplocal";
     return CUBE_ERR_PARAM;
   }
@@ -427,6 +439,7 @@ int32_t cube_load_state(cube_ctx* ctx, int64_t nplocal, const void* xp, const vo
   };
   auto copy = [&]() -> int {
     int rc;
+    if (add_here && (rc = counts(nullptr))) return rc;
     if ((rc = codes(xp, ctx->slot_r2, ctx->xp2, ctx->izipx))) return rc;  // 8 bytes per particle of scratch each
     if ((rc = codes(vp, ctx->slot_s2, ctx->vp2, ctx->izipv))) return rc;
     if (pid) CUBE_CUDA_TRY(ctx, cudaMemcpyAsync(ctx->pid2, pid, 4 * np, cudaMemcpyHostToDevice, st));

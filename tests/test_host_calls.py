@@ -78,13 +78,15 @@ print(json.dumps(calls()))
     assert len(streams) == 1 and streams != {"(nil)"}, [c for c in log if c["stream"] == "(nil)"]
 
 
-def test_contradicting_counts_are_refused_before_the_particle_arrays_are_read(child):
+@pytest.mark.parametrize("nc", [16, 40])  # 2^14 cells and fewer are added on the host, more on the device
+def test_contradicting_counts_are_refused_before_the_particle_arrays_are_read(child, nc):
     """A caller whose particle count is larger than its arrays (the kernels do nothing here: the
     device's total stays 0 against 64)."""
-    code, read, log = child("""
-g = empty_box()
+    code, read, log = child(f"""
+nc = {nc}
+g = Cube(make_params(nc, 2), np_capacity=64)
 xp, vp, pid = np.zeros((64, 3), np.int16), np.zeros((64, 3), np.int16), np.zeros(64, np.int32)
-rhoc, vf = np.zeros(16 ** 3, np.int32), np.zeros((16 ** 3, 3), np.float32)
+rhoc, vf = np.zeros(nc ** 3, np.int32), np.zeros((nc ** 3, 3), np.float32)
 fake.fake_clear()
 try:
     g.load_state(xp, vp, pid, rhoc, vf)
@@ -96,7 +98,7 @@ n = sum(c["name"] == "h2d" for c in calls())
 print(json.dumps([code, [any(read[i * n:(i + 1) * n]) for i in range(5)], calls()]))
 """)
     assert code == 1
-    assert read == [False] * 4 + [True], log
+    assert read == [False] * 4 + [nc == 40], log
 
 
 @pytest.mark.parametrize("short", range(5))
