@@ -132,9 +132,11 @@ int32_t cube_create(const cube_params* params, int64_t np_capacity,
                     const float* fk_table, const float* ck_table, cube_ctx** out);
 
 /* Copies a checkpoint-layout state to the device (particle_initialization.f90:34-82).
- * Load (and store) between steps, after cube_particle_mesh, where the reference
- * reads and writes checkpoints: a state loaded between cube_update_x and
- * cube_particle_mesh was measured to change the run that follows. */
+ * The reference reads and writes checkpoints between steps, after cube_particle_mesh;
+ * stored and loaded again between cube_update_x and cube_particle_mesh a state goes
+ * on bit for bit too, also after other states were stepped on the context meanwhile.
+ * CUBE_ERR_PARAM if the counts rhoc do not add up to nplocal (before the other arrays
+ * are read); after any error the state that was there is there still. */
 int32_t cube_load_state(cube_ctx* ctx, int64_t nplocal, const void* xp, const void* vp,
                         const int32_t* pid, const int32_t* rhoc, const float* vfield);
 
