@@ -226,7 +226,7 @@ def nu_params_for(cfg):
 # by 8 from c2s to c2 (and the fine mesh is the same in c3), so these scale with the
 # particle count; phases without a capture of every kernel have none.
 TRAFFIC_C2S = {"fine_fft_green": (0.537 + 0.492) + 4 * (0.539 + 0.492) + (0.743 + 1.568) + (1.711 + 1.554),
-               "kick": 1.894 + 0.100, "deposit": 0.135 + 0.498}  # GB per step at 256^3 particles
+               "kick": 1.890 + 0.100, "deposit": 0.135 + 0.498}  # GB per step at 256^3 particles
 
 
 def phase_traffic(config, phase, npart):
